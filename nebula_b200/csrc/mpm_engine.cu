@@ -645,11 +645,12 @@ void MPMEngine::uploadState(const float* const f[8], uint32_t n) {
 }
 
 // The state buffer holding the current particles in their original order:
-// the current buffer, or the idle one after an unpermute (once per state version).
+// the current buffer, or the idle one after an unpermute (once per state
+// version; every time once a caller's graph holds a step).
 StatePtrs MPMEngine::originalOrder() {
   if (!permuted_ || !live_) return statePtrs(cur_);
   StatePtrs tmp = statePtrs(cur_ ^ 1);  // free between substeps
-  if (unpermutedVersion_ != stateVersion_) {
+  if (inCallersGraph_ || unpermutedVersion_ != stateVersion_) {
     check(launchUnpermute(statePtrs(cur_), static_cast<const uint32_t*>(pid_[cur_].ptr), tmp, live_, lastStream_, &launches_), "unpermute");
     unpermutedVersion_ = stateVersion_;
   }
@@ -897,6 +898,7 @@ void MPMEngine::step(float dt, cudaStream_t s) {
     quiesce();
     lastStream_ = s;
   }
+  if (!inCallersGraph_) inCallersGraph_ = streamCapturing(s);
   // the emitters run first (MPMEngine.cpp:406); new particles invalidate the pending P2G
   if (!emitters_.empty() && emitFromEmitters(dt, s)) discardPending(s);
   const int n = std::max(1, params_.numSubsteps);
@@ -958,15 +960,18 @@ std::vector<unsigned char> MPMEngine::graphKey(const SubstepParams& P) {
   return k;
 }
 
-bool MPMEngine::graphsUsable(cudaStream_t s) const {
-  if (!useGraphs_ || profile_) return false;
-  // inside a capture of the caller's the launches go into the caller's graph
+bool streamCapturing(cudaStream_t s) {
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
     (void)cudaGetLastError();
-    return false;
+    return true;
   }
-  return st == cudaStreamCaptureStatusNone;
+  return st != cudaStreamCaptureStatusNone;
+}
+
+bool MPMEngine::graphsUsable(cudaStream_t s) const {
+  // inside a capture of the caller's the launches go into the caller's graph
+  return useGraphs_ && !profile_ && !streamCapturing(s);
 }
 
 void MPMEngine::clearGraphs() {

@@ -48,6 +48,10 @@ void domainGridRes(const float size[3], float h, uint32_t out[3]);
 uint32_t domainCubeRes(const uint32_t res[3]);
 uint32_t domainHashCells(const uint32_t res[3]);
 
+// True while `s` records into a graph (or when that cannot be found out): work
+// queued now runs when a caller replays it, without a call to the engine.
+bool streamCapturing(cudaStream_t s);
+
 // Owning device allocation.
 struct DevBuf {
   void* ptr = nullptr;
@@ -231,9 +235,12 @@ class MPMEngine {
   int cur_ = 0;
   bool permuted_ = false;
   // Bumped by every change of the particle state; the idle state buffer holds
-  // the original-order copy of version unpermutedVersion_ (downloads reuse it).
+  // the original-order copy of version unpermutedVersion_ (downloads reuse it,
+  // unless a caller's graph holds a step: its replays change the state, and the
+  // idle buffer, without a call here).
   uint64_t stateVersion_ = 0;
   uint64_t unpermutedVersion_ = ~uint64_t(0);
+  bool inCallersGraph_ = false;
   int pipeline_ = NEBULA_MPM_PIPELINE_FUSED;
   LaunchConfig launchCfg_;
   int numSMs_ = 148;
