@@ -91,6 +91,7 @@ class BatchEngine {
   int cur_ = 0;
   bool permuted_ = false;
   bool unpermuted_ = false;  // the idle state buffer holds the particles in original order (until the next step)
+  bool inCallersGraph_ = false;  // a step was recorded into a graph of the caller's: replays move the state without a call
   DevBuf gridAcc_, gridVel_, gridVold_;
   DevBuf bCount_, bFlag_, bStart_, cCount_[2], pbBrick_, pbStart_, gbBrick_, counters_, scanState_, scanTile_, binKey_, binRank_, perm_, err_;
   uint32_t tiles_ = 1;

@@ -150,6 +150,75 @@ def test_dt_change_and_host_edits_between_steps():
         assert rel_l2(Fm(got), Fm(want)) < 1e-4
 
 
+@pytest.mark.parametrize("graphs", [True, False])
+@pytest.mark.parametrize("substeps", [5, 6])
+def test_batch_read_back_follows_steps_and_edits(graphs, substeps):
+    """Read back, step, read back again, replace one scene's state, read back,
+    step, read back: every read-back is of its own time (a step of an odd and of
+    an even number of substeps, replayed and eager), as the single-scene engine
+    gives it."""
+    scenes = small_mix(n=3)
+    dt = scenes[0].params.dt
+    b, ids = batch_for_scenes(scenes)
+    b.set_graphs(graphs)
+    stream = torch.cuda.Stream()
+    plain = [engine_for_scene(sc) for sc in scenes]
+    for sc, s, p in zip(scenes, ids, plain):
+        b.set_collider_track(s, S.collider_track(sc, 1))
+        p.setColliderTrack(S.collider_track(sc, 1))
+
+    def check(what):
+        for s, p in zip(ids, plain):
+            got, want = b.state(s), p.state()
+            assert rel_l2(got["P"][:, :3], want["P"][:, :3]) < 1e-5, what
+            assert rel_l2(Fm(got), Fm(want)) < 1e-4, what
+
+    for k in range(3):
+        b.run_substeps(dt, substeps, stream=stream)
+        for p in plain:
+            p.run_substeps(dt, substeps)
+        check("step %d" % k)
+    st = plain[1].state()
+    st["P"][:, 0] += np.float32(2 * scenes[1].params.cell_size)
+    b.upload_state(ids[1], st)
+    plain[1].upload_state(st)
+    check("edit")
+    b.run_substeps(dt, substeps, stream=stream)
+    for p in plain:
+        p.run_substeps(dt, substeps)
+    check("step after the edit")
+
+
+def test_batch_read_back_between_replays_of_a_callers_graph():
+    """A step captured into a graph of the caller's (with the batch's own graphs
+    off: CUDA refuses to launch one into a capture) moves the state without a
+    call to the batch: read-backs after each of three replays against a batch
+    stepped eagerly."""
+    scenes = small_mix(n=3)
+    dt = scenes[0].params.dt
+    (a, ids), (e, _) = batch_for_scenes(scenes), batch_for_scenes(scenes)
+    stream = torch.cuda.Stream()
+    for b in (a, e):
+        b.set_graphs(False)
+        for sc, s in zip(scenes, ids):
+            b.set_collider_track(s, S.collider_track(sc, 1))
+        b.run_substeps(dt, 6, stream=stream)
+        b.sync()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream):
+        with torch.cuda.graph(g, stream=stream):
+            a.run_substeps(dt, 6, stream=stream)
+        for k in range(3):
+            g.replay()
+            torch.cuda.synchronize()
+            e.run_substeps(dt, 6, stream=stream)
+            e.sync()
+            for s in ids:
+                x, y = a.state(s), e.state(s)
+                assert rel_l2(x["P"][:, :3], y["P"][:, :3]) < 1e-6, k
+                assert rel_l2(Fm(x), Fm(y)) < 1e-5, k
+
+
 def test_batch_errors():
     b = BatchEngine(2, 1000)
     cfg = MPMConfig(nx=0, ny=0, nz=0, domainSize=(1, 1, 1), cellSize=1 / 32, maxParticles=0)
