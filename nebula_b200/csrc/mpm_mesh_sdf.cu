@@ -17,7 +17,9 @@
 // computes a closest point:
 //   1. U = min over triangles and their vertices of the distance from the
 //      vertex to the farthest cell centre of the box.  Every cell of the box
-//      has a triangle within U, so its closest distance is <= U.
+//      has a triangle within U, so its closest distance is <= U.  A triangle
+//      that may never be closest (a vertex that is not finite, hardly any area)
+//      bounds nothing.
 //   2. The triangles are staged through shared memory in tiles of 256, in
 //      list order.  A triangle whose bounding sphere is farther than U from
 //      the box cannot be any cell's closest and is dropped from the tile; the
@@ -192,6 +194,30 @@ __device__ __forceinline__ float discBound(const Disc& d, float px, float py, fl
   return sqrtf(l * l + o * o) * (1.0f - 1e-6f) + (nan == nan ? 0.f : nan);
 }
 
+// Whether a (posed) triangle is sure to be as close as its vertices: nine finite
+// coordinates and some area.  (A NaN or an overflow fails the comparison.  With a
+// NaN the closest point is NaN; without area the region test may return any
+// point of the plane.)
+__device__ __forceinline__ bool canBeClosest(const float (&v)[12]) {
+  const float ax = v[6] - v[3], ay = v[7] - v[4], az = v[8] - v[5], cx = v[9] - v[3], cy = v[10] - v[4], cz = v[11] - v[5];
+  const float gx = ay * cz - az * cy, gy = az * cx - ax * cz, gz = ax * cy - ay * cx;
+  const float e2 = dot3f(ax, ay, az, ax, ay, az) + dot3f(cx, cy, cz, cx, cy, cz);
+  return dot3f(gx, gy, gz, gx, gy, gz) > 1e-6f * e2 * e2;
+}
+
+// Squared distance from the triangle's nearest vertex to the farthest point of a box.
+__device__ __forceinline__ float farthestCell2(const float (&v)[12], float lox, float loy, float loz, float hix, float hiy, float hiz) {
+  float m2 = INFINITY;
+#pragma unroll
+  for (int j = 1; j < 4; ++j) {
+    const float ex = fmaxf(v[3 * j] - lox, hix - v[3 * j]);
+    const float ey = fmaxf(v[3 * j + 1] - loy, hiy - v[3 * j + 1]);
+    const float ez = fmaxf(v[3 * j + 2] - loz, hiz - v[3 * j + 2]);
+    m2 = fminf(m2, ex * ex + ey * ey + ez * ez);
+  }
+  return m2;
+}
+
 __global__ void __launch_bounds__(kThreads) k_mesh_sdf(const float4* __restrict__ tris, uint32_t n, MeshPose pose, int rx, int ry, int rz,
                                                        uint32_t totalCells, float cs, float eps, float* __restrict__ sdf) {
   __shared__ TriS tile[kThreads];
@@ -214,15 +240,26 @@ __global__ void __launch_bounds__(kThreads) k_mesh_sdf(const float4* __restrict_
   if (threadIdx.x == 0) boundBits = __float_as_uint(INFINITY);
   __syncthreads();
   float u2 = INFINITY;
+  uint32_t nearest = n;
   for (uint32_t k = threadIdx.x; k < n; k += kThreads) {
     float v[12];
     loadTri(tris, k, pose, v);
-#pragma unroll
-    for (int j = 1; j < 4; ++j) {
-      const float ex = fmaxf(v[3 * j] - lox, hix - v[3 * j]);
-      const float ey = fmaxf(v[3 * j + 1] - loy, hiy - v[3 * j + 1]);
-      const float ez = fmaxf(v[3 * j + 2] - loz, hiz - v[3 * j + 2]);
-      u2 = fminf(u2, ex * ex + ey * ey + ez * ez);
+    const float m2 = farthestCell2(v, lox, loy, loz, hix, hiy, hiz);
+    if (m2 < u2) {
+      u2 = m2;
+      nearest = k;
+    }
+  }
+  // a triangle that may never be closest bounds nothing: if the nearest is one, once more without them
+  if (nearest < n) {
+    float v[12];
+    loadTri(tris, nearest, pose, v);
+    if (!canBeClosest(v)) {
+      u2 = INFINITY;
+      for (uint32_t k = threadIdx.x; k < n; k += kThreads) {
+        loadTri(tris, k, pose, v);
+        if (canBeClosest(v)) u2 = fminf(u2, farthestCell2(v, lox, loy, loz, hix, hiy, hiz));
+      }
     }
   }
   u2 = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(u2)));  // non-negative floats order as their bits

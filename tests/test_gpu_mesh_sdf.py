@@ -275,11 +275,27 @@ def test_prepared_tree_equals_list_kernel(count, pose):
     tris[5, 7] = np.nan
     res = (24, 20, 17)
     total = S.hash_cells(res)
-    # (without the NaN triangle: the list kernel takes bounds from its other vertices)
-    a = gpu_mesh_sdf(np.delete(tris, 5, axis=0), res, total, 1.0 / 24, prepared=False, t=t, q=q)
+    a = gpu_mesh_sdf(tris, res, total, 1.0 / 24, prepared=False, t=t, q=q)
     b = gpu_mesh_sdf(tris, res, total, 1.0 / 24, prepared=True, t=t, q=q)
     tol = 1e-5 + (900 * 6e-8 * 20 if pose and abs(t[0]) > 10 else 0.0)
     assert np.abs(np.abs(a) - np.abs(b)).max() <= tol
     far = np.abs(a) > 2 * tol
     # two triangles of the soup may be equally near with opposite normals: their sign is the tie rule's, up to rounding
     assert (np.sign(a[far]) != np.sign(b[far])).mean() <= 1e-3
+
+
+@pytest.mark.parametrize("prepared", [False, True])
+def test_triangle_with_a_nan_vertex_bounds_nothing(prepared):
+    """A triangle with a NaN vertex is closest to no cell, and its two other
+    vertices, far from the mesh, must not keep the mesh from the cells around
+    them (list lengths below and above one per thread of a CTA)."""
+    res, total, h = (32, 32, 32), 32 ** 3, 1 / 32
+    tri = np.array([[0, 1, 0, 0.8, 0.8, 0.8, 0.82, 0.8, 0.8, 0.8, 0.8, 0.82]], np.float32)
+    for subdivisions in (1, 2):
+        base = mesh.icosphere((0.2, 0.2, 0.2), 0.1, subdivisions)
+        want = oracle.mesh_sdf(base, res, total, h)
+        for vertex in range(3):
+            t = tri.copy()
+            t[0, 4 + 3 * vertex] = np.nan
+            for at in (0, len(base)):
+                assert_same_sdf(gpu_mesh_sdf(np.insert(base, at, t, axis=0), res, total, h, prepared), want)
