@@ -180,7 +180,8 @@ __device__ __forceinline__ void g2pGather(const SubstepParams& P, const PState& 
   const float xp[3] = {s.P.x, s.P.y, s.P.z};
   int base[3];
 #pragma unroll
-  for (int a = 0; a < 3; ++a) base[a] = int(floorf(__fdiv_rn(xp[a] - P.worldMin[a], h))) - 1;
+  for (int a = 0; a < 3; ++a)  // (a cell farther out than the clamp has no node on the grid either)
+    base[a] = max(min(__float2int_rd(__fdiv_rn(xp[a] - P.worldMin[a], h)), P.gridRes[a] + 1), -2) - 1;
   const bool flip = P.flip_ratio > 0.01f;
 #pragma unroll
   for (int i = 0; i < 3; ++i) vpic[i] = vpo[i] = 0.f;
@@ -237,21 +238,24 @@ __device__ __forceinline__ void g2pGather(const SubstepParams& P, const PState& 
 // the node is lighter than 1e-10 -- exactly the nodes the shader skips.  The
 // B-spline weights are products of 1D factors, so sums run along x first for
 // each (dy, dz) and are then scaled by the y/z factors.  cx, cy, cz receive the
-// particle's cell.  Returns false when the particle's stencil is not inside
-// [0, gridRes) (the caller then uses g2pGather).
+// particle's cell, clamped to the grid as the binning clamps it.  Returns false
+// when the particle's stencil is not inside [0, gridRes) (the caller then uses
+// g2pGather).
 template <bool FLIP>
 __device__ __forceinline__ bool g2pGatherGrid(const SubstepParams& P, const PState& s, const float4* gv, const float4* gvo,
                                               float vpic[3], float vpo[3], float G[3][3], float Bn[3][3], int& cx, int& cy, int& cz) {
   const float h = P.cellSize, invH = 1.0f / P.cellSize;
   const float xp[3] = {s.P.x, s.P.y, s.P.z};
-  int base[3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a) base[a] = int(floorf(__fdiv_rn(xp[a] - P.worldMin[a], h))) - 1;
-  cx = base[0] + 1;
-  cy = base[1] + 1;
-  cz = base[2] + 1;
-  if (base[0] < 0 || base[1] < 0 || base[2] < 0 || base[0] > P.gridRes[0] - 3 || base[1] > P.gridRes[1] - 3 || base[2] > P.gridRes[2] - 3)
+  cx = __float2int_rd(__fdiv_rn(xp[0] - P.worldMin[0], h));  // (saturates; NaN: 0)
+  cy = __float2int_rd(__fdiv_rn(xp[1] - P.worldMin[1], h));
+  cz = __float2int_rd(__fdiv_rn(xp[2] - P.worldMin[2], h));
+  if (cx < 1 || cy < 1 || cz < 1 || cx > P.gridRes[0] - 2 || cy > P.gridRes[1] - 2 || cz > P.gridRes[2] - 2) {
+    cx = max(min(cx, P.gridRes[0] - 1), 0);
+    cy = max(min(cy, P.gridRes[1] - 1), 0);
+    cz = max(min(cz, P.gridRes[2] - 1), 0);
     return false;
+  }
+  const int base[3] = {cx - 1, cy - 1, cz - 1};
   uint32_t mx[3], my[3], mz[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {

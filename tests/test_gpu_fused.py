@@ -165,8 +165,8 @@ def test_fused_flip_and_pic_vs_oracle():
 
 
 def test_fused_fast_particle_leaves_tile():
-    """A FLIP particle crossing several cells per substep scatters outside its
-    block tile (global-reduction path) and still matches the oracle."""
+    """A FLIP particle crossing several cells per substep leaves the cells
+    around its brick, is counted, and still matches the oracle."""
     sp = S.StepParams(dt=5e-3, cell_size=1.0 / 16, domain_size=(1.0, 1.0, 1.0), flip_ratio=1.0,
                       materials=[S.material(S.MAT_ELASTIC, 1e3, 0.3, 1000.0)], forces=[])
     pos = np.array([[0.3, 0.5, 0.5], [0.5, 0.5, 0.5]], np.float32)
@@ -179,6 +179,24 @@ def test_fused_fast_particle_leaves_tile():
     rs = oracle_run(sc, 4)
     assert rel_l2(gs["P"][:, :3], rs["P"][:, :3]) < 1e-6
     assert rel_l2(gs["v"][:, :3], rs["v"][:, :3]) < 1e-5
+
+
+@pytest.mark.parametrize("x", [-0.1, 1.2, -1e12, 1e12])
+def test_particle_from_outside_the_domain_is_not_counted_as_a_leaver(x):
+    """A particle uploaded outside the domain is binned in the border cell and
+    put back beside it by the position clamp of its first substep: it has not
+    left the cells around its brick, however far outside it was."""
+    sp = S.StepParams(dt=1e-4, cell_size=1.0 / 16, domain_size=(1.0, 1.0, 1.0), flip_ratio=-1.0,
+                      materials=[S.material(S.MAT_ELASTIC, 1e3, 0.3, 1000.0)], forces=[])
+    for axis in range(3):
+        pos = np.full((2, 3), 0.5, np.float32)
+        pos[0, axis] = x
+        eng = engine_for_scene(S.Scene("outside", sp, S.make_state(pos, np.float32(1e-4), vel=np.zeros((2, 3), np.float32)), 8))
+        eng.run_substeps(sp.dt, 2)
+        eng.sync()
+        p = eng.state()["P"]
+        assert np.all((p[:, :3] > 0) & (p[:, :3] < 1))
+        assert eng.stats()["overflow_particles"] == 0
 
 
 def test_fused_export_grid_after_step_is_p2g_of_state():
