@@ -35,7 +35,11 @@ from typing import Callable, Iterable
 from . import _capi
 
 CACHE_ENV = "NEBULA_B200_TUNE_CACHE"
-CACHE_VERSION = 3  # 2: shapes carry fused_split; 3: 192-thread CTAs, contiguous brick parts
+# Raised whenever shapes change their meaning, so that none is applied to a
+# kernel it was not measured on.  2: shapes carry fused_split; 3: 192-thread CTAs,
+# contiguous brick parts; 4: the fused kernel takes rounds of 32 particles per
+# warp, in CTAs of 1 to 8 warps by scene size when the shape leaves that open.
+CACHE_VERSION = 4
 
 
 @dataclass(frozen=True)

@@ -70,6 +70,17 @@ def test_damaged_cache_is_replaced(tmp_path):
     assert rep["source"] == "measured" and json.loads(path.read_text())["entries"]["k"]["shape"]["fused_threads"] == 192
 
 
+def test_shapes_of_an_older_kernel_are_not_applied(tmp_path):
+    """A cache written before the fused kernel changed (any other version) is
+    measured again, not applied."""
+    path = tmp_path / "shapes.json"
+    old = {"shape": {"fused_threads": 192, "fused_ctas_per_sm": 3, "grid_ctas_per_sm": 0, "grid_batch": 4, "fused_split": 2}}
+    for version in (2, 3, None):
+        path.write_text(json.dumps({"version": version, "entries": {"k": old}}))
+        best, rep = A.tune(lambda s: 1.0 if s == A.LaunchShape() else 2.0, "k", LIM, path, repeats=1)
+        assert rep["source"] == "measured" and best == A.LaunchShape()
+
+
 def test_keys_and_shape_conversions(tmp_path, monkeypatch):
     k = A.workload_key("batch", 3_140_220, 128, False, [2, 0, 2], 64)
     assert k == "batch|n2^22|cube128|pic-apic|models0-2|scenes64"
