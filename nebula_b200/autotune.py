@@ -2,18 +2,18 @@
 
 The fused G2P/P2G kernel and the grid update take their launch shape from a
 ``nebula_mpm_launch_config``: the fused kernel's CTA size (192 or 256 threads),
-how many persistent CTAs each of the two kernels keeps per SM, the grid
-kernel's nodes per thread per round (2 or 4), and into how many work items
-the fused kernel cuts a particle brick (1-4).  Which shape is
-fastest depends on the GPU and on the workload (particles per brick, scene
-sizes, FLIP or APIC, the material mix), so ``tune`` times candidate shapes on
-the caller's own workload with CUDA events and keeps the fastest, by
-coordinate descent in three rounds (the fused kernel's CTA shape, its items
-per brick, then the grid update's shape), and stores the result in a JSON
-cache keyed by the GPU and a
-workload key; a later run on the same GPU and workload reuses the entry
-without timing anything.  Every shape computes the same substep (float sums
-may associate differently), so tuning changes speed, not results.
+how many persistent CTAs each of the two kernels keeps per SM, and the grid
+kernel's nodes per thread per round (2 or 4).  Which shape is fastest depends
+on the GPU and on the workload (particles per brick, scene sizes, FLIP or APIC,
+the material mix), so ``tune`` times candidate shapes on the caller's own
+workload with CUDA events and keeps the fastest, by coordinate descent (the
+fused kernel's CTA shape, then the grid update's shape), and stores the result
+in a JSON cache keyed by the GPU and a workload key; a later run on the same GPU
+and workload reuses the entry without timing anything.  Every shape computes
+the same substep (float sums may associate differently), so tuning changes
+speed, not results.  ``fused_split`` is accepted and kept by the engine without
+effect, so ``tune_engine`` and ``tune_batch`` leave it at 0; ``tune`` tries its
+values, as a round between the two, for a ``measure`` of the caller's own.
 
     shape, report = tune_engine(engine, scene)          # applied to `engine`
     shape, report = tune_batch(batch, scenes, ids)      # applied to `batch`
@@ -159,10 +159,11 @@ def device_key() -> str:
 
 
 def tune(measure: Callable[[LaunchShape], float], key: str, limits: Limits, path=None, force: bool = False, repeats: int = 2,
-         base: LaunchShape = LaunchShape()) -> tuple[LaunchShape, dict]:
+         base: LaunchShape = LaunchShape(), splits: bool = True) -> tuple[LaunchShape, dict]:
     """The fastest shape by `measure` (ms per substep of one shape; called
     `repeats` times per candidate, the minimum kept).  A cached entry under
-    `key` is returned unless `force`."""
+    `key` is returned unless `force`.  `splits`: try the values of fused_split
+    too (they are all the same to the engine's kernels)."""
     p = cache_path(path)
     if not force:
         hit = _load(p)["entries"].get(key)
@@ -179,7 +180,8 @@ def tune(measure: Callable[[LaunchShape], float], key: str, limits: Limits, path
 
     t_base = timed(base)
     best = min(fused_candidates(base, limits), key=timed)
-    best = min(split_candidates(best), key=timed)
+    if splits:
+        best = min(split_candidates(best), key=timed)
     best = min(grid_candidates(best, limits), key=timed)
     entry = {"shape": asdict(best), "ms_per_substep": seen[best], "default_ms_per_substep": t_base,
              "tried": [[asdict(s), t] for s, t in tried], "when": time.strftime("%Y-%m-%dT%H:%M:%S")}
@@ -214,7 +216,7 @@ def tune_engine(eng, scene, substeps: int = 10, path=None, force: bool = False, 
         eng.sync()
         return _events_ms(lambda: eng.run_substeps(sp.dt, substeps, stream), stream) / substeps
 
-    shape, rep = tune(measure, key, device_limits(flip, False), path, force, repeats)
+    shape, rep = tune(measure, key, device_limits(flip, False), path, force, repeats, splits=False)
     eng.set_launch_config(shape)
     if rep["source"] == "measured":
         eng.upload_state(scene.state)
@@ -244,7 +246,7 @@ def tune_batch(batch, scenes, ids, substeps: int = 20, path=None, force: bool = 
         batch.sync()
         return _events_ms(lambda: batch.step(dt * substeps, substeps, stream), stream) / substeps
 
-    shape, rep = tune(measure, key, device_limits(flip, True), path, force, repeats)
+    shape, rep = tune(measure, key, device_limits(flip, True), path, force, repeats, splits=False)
     batch.set_launch_config(shape)
     if rep["source"] == "measured":
         restore()

@@ -81,6 +81,29 @@ def test_shapes_of_an_older_kernel_are_not_applied(tmp_path):
         assert rep["source"] == "measured" and best == A.LaunchShape()
 
 
+def test_engine_tuning_leaves_the_split_alone(tmp_path, monkeypatch):
+    """fused_split has no effect on the engine's kernels: tune_engine and
+    tune_batch neither time its values nor store one that noise preferred."""
+    seen = []
+    real = A.tune
+    monkeypatch.setattr(A, "tune", lambda measure, key, lim, *a, **k: real(lambda s: seen.append(s) or cost(s), key, LIM, *a, **k))
+    monkeypatch.setattr(A, "device_limits", lambda flip, batch: LIM)
+    monkeypatch.setattr(A, "device_key", lambda: "gpu")
+    import torch
+    monkeypatch.setattr(torch.cuda, "Stream", lambda: None)
+
+    class Fake:
+        def __getattr__(self, name):
+            return lambda *a, **k: None
+
+    from nebula_b200 import scenes as S
+    sc = S.shear_block()
+    for k, run in enumerate((lambda p: A.tune_engine(Fake(), sc, path=p), lambda p: A.tune_batch(Fake(), [sc], [0], path=p))):
+        shape, rep = run(tmp_path / ("%d.json" % k))
+        assert shape == A.LaunchShape(192, 3, 4, 2, 0) and rep["source"] == "measured"
+    assert {s.fused_split for s in seen} == {0}
+
+
 def test_keys_and_shape_conversions(tmp_path, monkeypatch):
     k = A.workload_key("batch", 3_140_220, 128, False, [2, 0, 2], 64)
     assert k == "batch|n2^22|cube128|pic-apic|models0-2|scenes64"
