@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(kThreads) k_mesh_sdf_discs(const float4* __res
                                                              const float4* __restrict__ discs, const float4* __restrict__ points, uint32_t n, uint32_t nLeaves, uint32_t nGroups,
                                                              uint32_t nBlocks, MeshPose pose, int rx, int ry, int rz, uint32_t totalCells, float cs,
                                                              float eps, float pad, float* __restrict__ sdf) {
-  constexpr uint32_t kFull = 0xffffffffu;
+  constexpr uint32_t kFull = 0xffffffffu, kTileLeaves = 32u / kMeshLeaf;
   __shared__ __align__(16) TriD tiles[kThreads];
   __shared__ uint32_t tileIdx[kThreads];
   const uint32_t code = blockIdx.x * kThreads + threadIdx.x;
@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(kThreads) k_mesh_sdf_discs(const float4* __res
   bool outer = true;
   float most = 1e9f;           // the lanes' largest bound
   uint32_t hot = 0, nHot = 0;  // collected leaves, one in each of the lanes 0..nHot-1
-  uint32_t near = 0xffffffffu;  // the leaf that gave the bound
+  uint32_t near = 0;           // the leaf that gave the bound
 
   auto tighten = [&]() { most = __uint_as_float(__reduce_max_sync(kFull, __float_as_uint(bound))); };
   // the distance to a vertex of leaf l
@@ -507,34 +507,52 @@ __global__ void __launch_bounds__(kThreads) k_mesh_sdf_discs(const float4* __res
     }
   };
 
-  // 1. the leaf nearest the box's centre
-  if (nBlocks) {
-    const uint32_t b = nearestDisc(discs, nLeaves + nGroups, nBlocks, cx, cy, cz);
-    const uint32_t g = b * kMeshFan + nearestDisc(discs, nLeaves + b * kMeshFan, min(kMeshFan, nGroups - b * kMeshFan), cx, cy, cz);
-    const uint32_t l = g * kMeshFan + nearestDisc(discs, g * kMeshFan, min(kMeshFan, nLeaves - g * kMeshFan), cx, cy, cz);
-    vertexBound(l);
-    tighten();
+  // Small meshes leave steps out, whose fixed cost per warp is most of their
+  // time.  Up to 32 triangles are one tile: no search (a soup of 4 on 128^3 108 ->
+  // 54 us, of 32 183 -> 145; the clusters with bounding spheres that the tree
+  // replaced took 95 and 201).  Up to a group of leaves, every leaf gives its
+  // bound, without the descent and the first walk (40 triangles 197 -> 157 us, the
+  // clusters 161; 300: 322 -> 294, the clusters 304); from there on the walk pays
+  // (450: 327 -> 322, 512: 345 -> 347).
+  if (nLeaves <= kTileLeaves) {
+    for (uint32_t l = 0; l < nLeaves; ++l) vertexBound(l);
+    hot = lane;
+    nHot = nLeaves;
+  } else {
+    if (nLeaves <= kMeshFan) {
+      // 1., 2. a bound per lane
+      for (uint32_t l = 0; l < nLeaves; ++l) vertexBound(l);
+      tighten();
+    } else {
+      // 1. the leaf nearest the box's centre
+      const uint32_t b = nearestDisc(discs, nLeaves + nGroups, nBlocks, cx, cy, cz);
+      const uint32_t g = b * kMeshFan + nearestDisc(discs, nLeaves + b * kMeshFan, min(kMeshFan, nGroups - b * kMeshFan), cx, cy, cz);
+      near = g * kMeshFan + nearestDisc(discs, g * kMeshFan, min(kMeshFan, nLeaves - g * kMeshFan), cx, cy, cz);
+      vertexBound(near);
+      tighten();
+      // 2. a bound per lane
+      walk(vertexBound, tighten);
+    }
+    // 3. the closest triangles: first the leaves that gave the bounds (the
+    // nearest leaf where no vertex may bound: a mesh of slivers)
+    auto collect = [&](uint32_t l) {
+      if (lane == nHot) hot = l;
+      if (++nHot == kTileLeaves) flush();
+    };
+    uint32_t todo = __ballot_sync(kFull, inside);
+    while (todo) {
+      const uint32_t l = __shfl_sync(kFull, near, __ffs(todo) - 1);
+      todo &= ~__ballot_sync(kFull, near == l);
+      collect(l);
+    }
+    if (nHot) flush();
+    walk(
+        [&](uint32_t l) {
+          if (__any_sync(kFull, inside && near == l)) return;  // done above
+          if (__any_sync(kFull, !discBeyond(loadDisc(discs, l), mx, my, mz, pad, bound))) collect(l);
+        },
+        [] {});
   }
-  // 2. a bound per lane
-  walk(vertexBound, tighten);
-  // 3. the closest triangles: first the leaves that gave the bounds
-  auto collect = [&](uint32_t l) {
-    if (lane == nHot) hot = l;
-    if (++nHot == 4u) flush();
-  };
-  uint32_t todo = __ballot_sync(kFull, inside && near < nLeaves);
-  while (todo) {
-    const uint32_t l = __shfl_sync(kFull, near, __ffs(todo) - 1);
-    todo &= ~__ballot_sync(kFull, near == l);
-    collect(l);
-  }
-  if (nHot) flush();
-  walk(
-      [&](uint32_t l) {
-        if (__any_sync(kFull, inside && near == l)) return;  // done above
-        if (__any_sync(kFull, !discBeyond(loadDisc(discs, l), mx, my, mz, pad, bound))) collect(l);
-      },
-      [] {});
   if (nHot) flush();
   if (code < totalCells) sdf[code] = inside ? (outer ? best : -best) : 1e9f;
 }

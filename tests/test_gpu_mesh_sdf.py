@@ -299,3 +299,35 @@ def test_triangle_with_a_nan_vertex_bounds_nothing(prepared):
             t[0, 4 + 3 * vertex] = np.nan
             for at in (0, len(base)):
                 assert_same_sdf(gpu_mesh_sdf(np.insert(base, at, t, axis=0), res, total, h, prepared), want)
+
+
+@pytest.mark.parametrize("count", [31, 32, 33, 64, 512, 513])
+def test_prepared_small_meshes_at_the_edges_of_their_paths(count):
+    """The largest mesh that is one tile, the smallest that is searched, the
+    largest of one group and one more, on a ragged grid with cells that the last
+    warps lack, against the oracle.  Every triangle comes twice with opposite
+    normals, so the tie rule shows as well (an odd count drops the last copy)."""
+    base = mesh.torus((0.5, 0.5, 0.5), 0.25, 0.08, 32, 16)[::2][: (count + 1) // 2]
+    flipped = base.copy()
+    flipped[:, 0:3] *= -1.0
+    tris = np.concatenate([flipped, base])[:count]
+    res = (21, 18, 13)
+    assert_same_sdf(gpu_mesh_sdf(tris, res, 32 ** 3, 1 / 21, True), oracle.mesh_sdf(tris, res, 32 ** 3, 1 / 21))
+
+
+@pytest.mark.parametrize("count", [40, 600])
+def test_prepared_mesh_of_slivers(count):
+    """Slivers, none of which may bound the others by its vertices (the area
+    rule): the search starts from the nearest leaf and still finds the closest."""
+    rng = np.random.default_rng(count)
+    a = rng.uniform(0.2, 0.8, (count, 3))
+    d, e = rng.normal(0.0, 1.0, (2, count, 3))
+    d *= 0.1 / np.linalg.norm(d, axis=1, keepdims=True)
+    v = np.stack([a, a + d, a + d + 3e-5 * e], 1)
+    nrm = np.cross(v[:, 1] - v[:, 0], v[:, 2] - v[:, 0])
+    nrm /= np.linalg.norm(nrm, axis=1, keepdims=True)
+    tris = np.concatenate([nrm[:, None], v], 1).reshape(count, 12).astype(np.float32)
+    res, total, h = (32, 32, 32), 32 ** 3, 1 / 32
+    got, want = gpu_mesh_sdf(tris, res, total, h, True), oracle.mesh_sdf(tris, res, total, h)
+    # the region test of a sliver 3e-5 wide may return any point across it: its width
+    assert np.abs(np.abs(got) - np.abs(want)).max() < 2e-4
