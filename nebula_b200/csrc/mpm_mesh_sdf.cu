@@ -33,7 +33,9 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <future>
 #include <memory>
+#include <system_error>
 #include <vector>
 
 #include "mpm_device.cuh"
@@ -712,36 +714,47 @@ cudaError_t launchMeshSdfPrepared(const PreparedMesh& m, const MeshPose& pose, c
 
 namespace {
 
-// Bounding disc of the vertices of sorted triangles [t0, t1): the plane of
-// their area-weighted normal through the middle of their bounding box.
-void hostDisc(const float* tris, uint32_t t0, uint32_t t1, float4* out) {
+// Bounding box, area-weighted normal and finiteness of a run of triangles.
+struct Extent {
   float l[3] = {INFINITY, INFINITY, INFINITY}, u[3] = {-INFINITY, -INFINITY, -INFINITY};
   double g[3] = {0.0, 0.0, 0.0};
-  bool finite = true;
-  for (uint32_t t = t0; t < t1; ++t) {
-    const float* v = tris + 12 * size_t(t) + 3;
-    for (int k = 0; k < 9; ++k) {
-      finite = finite && std::isfinite(v[k]);
-      l[k % 3] = std::min(l[k % 3], v[k]);
-      u[k % 3] = std::max(u[k % 3], v[k]);
-    }
-    double e[2][3];
-    for (int a = 0; a < 3; ++a) {
-      e[0][a] = double(v[3 + a]) - v[a];
-      e[1][a] = double(v[6 + a]) - v[a];
-    }
-    for (int a = 0; a < 3; ++a) g[a] += e[0][(a + 1) % 3] * e[1][(a + 2) % 3] - e[0][(a + 2) % 3] * e[1][(a + 1) % 3];
+  float bad = 0.f;  // NaN when a coordinate is not finite
+  void add(const float* v) {
+    for (int k = 0; k < 9; k += 3)
+      for (int a = 0; a < 3; ++a) {
+        bad += v[k + a] * 0.f;
+        l[a] = std::min(l[a], v[k + a]);
+        u[a] = std::max(u[a], v[k + a]);
+      }
+    const double x1 = double(v[3]) - v[0], y1 = double(v[4]) - v[1], z1 = double(v[5]) - v[2];
+    const double x2 = double(v[6]) - v[0], y2 = double(v[7]) - v[1], z2 = double(v[8]) - v[2];
+    g[0] += y1 * z2 - z1 * y2;
+    g[1] += z1 * x2 - x1 * z2;
+    g[2] += x1 * y2 - y1 * x2;
   }
-  if (!finite) {  // never skipped
+  void add(const Extent& e) {
+    bad += e.bad;
+    for (int a = 0; a < 3; ++a) {
+      l[a] = std::min(l[a], e.l[a]);
+      u[a] = std::max(u[a], e.u[a]);
+      g[a] += e.g[a];
+    }
+  }
+};
+
+// Bounding disc of the vertices of sorted triangles [t0, t1): the plane of
+// their area-weighted normal through the middle of their bounding box.
+void hostDisc(const float* tris, uint32_t t0, uint32_t t1, const Extent& e, float4* out) {
+  if (e.bad != 0.f) {  // never skipped
     out[0] = make_float4(NAN, NAN, NAN, NAN);
     out[1] = make_float4(0.f, 0.f, 0.f, NAN);
     return;
   }
-  const double len = std::sqrt(g[0] * g[0] + g[1] * g[1] + g[2] * g[2]);
+  const double len = std::sqrt(e.g[0] * e.g[0] + e.g[1] * e.g[1] + e.g[2] * e.g[2]);
   float n[3], c[3];
   for (int a = 0; a < 3; ++a) {
-    c[a] = 0.5f * l[a] + 0.5f * u[a];
-    n[a] = len > 1e-30 && std::isfinite(len) ? float(g[a] / len) : 0.f;
+    c[a] = 0.5f * e.l[a] + 0.5f * e.u[a];
+    n[a] = len > 1e-30 && std::isfinite(len) ? float(e.g[a] / len) : 0.f;
   }
   double r2 = 0.0, th = 0.0;
   for (uint32_t t = t0; t < t1; ++t)
@@ -757,44 +770,81 @@ void hostDisc(const float* tris, uint32_t t0, uint32_t t1, float4* out) {
   out[1] = make_float4(n[0], n[1], n[2], float(th) * 1.0001f + slack);
 }
 
-}  // namespace
+constexpr size_t kForkTriangles = 8192;  // a split below this takes less than starting a thread is worth
+
+struct Centroid {
+  float c[3];
+  uint32_t index;  // in the caller's list
+  // position along an axis, ties by list index: unsigned integers order as the pairs
+  uint64_t key(int axis) const {
+    const float f = c[axis] + 0.0f;  // (-0 and 0 are one place)
+    uint32_t u;
+    std::memcpy(&u, &f, sizeof(u));
+    u ^= (u >> 31) ? 0xffffffffu : 0x80000000u;
+    return (uint64_t(u) << 32) | index;
+  }
+};
+
+// The mid - lo smallest of t[lo, hi) along an axis to the front, as
+// std::nth_element, by partitions without a branch per element: the comparisons
+// are unpredictable and were most of the preparation.
+void selectFront(std::vector<Centroid>& t, size_t lo, size_t mid, size_t hi, int axis) {
+  for (int rounds = 0; hi - lo > 16 && rounds < 64; ++rounds) {
+    uint64_t s[9];  // the pivot is the median of nine
+    for (size_t k = 0; k < 9; ++k) s[k] = t[lo + (hi - 1 - lo) * k / 8].key(axis);
+    std::sort(s, s + 9);
+    size_t m = lo;
+    for (size_t i = lo; i < hi; ++i) {
+      const Centroid c = t[i];
+      t[i] = t[m];
+      t[m] = c;
+      m += c.key(axis) < s[4] ? 1u : 0u;
+    }
+    if (m == mid) return;
+    if (mid < m) hi = m;
+    else lo = m;
+  }
+  std::nth_element(t.begin() + lo, t.begin() + mid, t.begin() + hi, [axis](const Centroid& p, const Centroid& q) { return p.key(axis) < q.key(axis); });
+}
 
 // Order of the triangles: median splits of the centroids along their longest
 // extent, cut at multiples of a block, then a group, then a leaf, so that the
 // runs of every level are compact.  (Runs of a Morton order jump between
 // distant patches of a surface and make wide leaves: 2.41 ms on the
 // 20,480-triangle sphere at 128^3, against 1.51.)
-// idx[t0, t1) of triangles with centroids `cen`; ties by list index, so the
-// order depends on the mesh alone.
-namespace {
-void orderTriangles(const std::vector<float>& cen, std::vector<uint32_t>& idx, size_t t0, size_t t1) {
+// t[t0, t1); ties by list index, so the runs depend on the mesh alone.  The
+// halves are independent: those of the first `forks` splits of a large mesh go to
+// threads of their own.
+void orderTriangles(std::vector<Centroid>& t, size_t t0, size_t t1, int forks) {
+  std::vector<std::future<void>> others;  // (joined on the way out)
   while (t1 - t0 > kMeshLeaf) {
     const size_t len = t1 - t0;
     size_t unit = kMeshLeaf;
     while (unit * kMeshFan < len) unit *= kMeshFan;
     const size_t mid = t0 + unit * (((len + unit - 1) / unit) / 2);
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (size_t t = t0; t < t1; ++t)
+    for (size_t k = t0; k < t1; ++k)
       for (int a = 0; a < 3; ++a) {
-        const float c = cen[3 * size_t(idx[t]) + a];
-        lo[a] = std::min(lo[a], c);
-        hi[a] = std::max(hi[a], c);
+        lo[a] = std::min(lo[a], t[k].c[a]);
+        hi[a] = std::max(hi[a], t[k].c[a]);
       }
     int axis = 0;
     for (int a = 1; a < 3; ++a)
       if (hi[a] - lo[a] > hi[axis] - lo[axis]) axis = a;
-    std::nth_element(idx.begin() + t0, idx.begin() + mid, idx.begin() + t1, [&](uint32_t p, uint32_t q) {
-      const float x = cen[3 * size_t(p) + axis], y = cen[3 * size_t(q) + axis];
-      return x < y || (x == y && p < q);
-    });
+    selectFront(t, t0, mid, t1, axis);
     // the larger half here, the smaller one below (the depth stays logarithmic)
-    if (mid - t0 < t1 - mid) {
-      orderTriangles(cen, idx, t0, mid);
-      t0 = mid;
-    } else {
-      orderTriangles(cen, idx, mid, t1);
-      t1 = mid;
+    const bool lower = mid - t0 < t1 - mid;
+    const size_t s0 = lower ? t0 : mid, s1 = lower ? mid : t1;
+    (lower ? t0 : t1) = mid;
+    if (forks > 0 && len >= kForkTriangles) {
+      --forks;
+      try {
+        others.push_back(std::async(std::launch::async, [&t, s0, s1, forks] { orderTriangles(t, s0, s1, forks); }));
+        continue;
+      } catch (const std::system_error&) {  // no thread to be had
+      }
     }
+    orderTriangles(t, s0, s1, forks);
   }
 }
 }  // namespace
@@ -805,28 +855,37 @@ void PreparedMesh::build(const float* h, uint32_t count) {
   leaves = (count + kMeshLeaf - 1) / kMeshLeaf;
   groups = (leaves + kMeshFan - 1) / kMeshFan;
   blocks = (groups + kMeshFan - 1) / kMeshFan;
-  std::vector<float> cen(size_t(count) * 3);
-  std::vector<uint32_t> idx(count);
+  std::vector<Centroid> cen(count);
   for (uint32_t k = 0; k < count; ++k) {
-    idx[k] = k;
+    cen[k].index = k;
     for (int a = 0; a < 3; ++a) {
       const float c = (h[12 * size_t(k) + 3 + a] + h[12 * size_t(k) + 6 + a] + h[12 * size_t(k) + 9 + a]) / 3.0f;
-      cen[3 * size_t(k) + a] = std::isfinite(c) ? c : 0.f;  // (any place: a triangle that is never closest)
+      cen[k].c[a] = std::isfinite(c) ? c : 0.f;  // (any place: a triangle that is never closest)
     }
   }
-  orderTriangles(cen, idx, 0, count);
+  orderTriangles(cen, 0, count, 3);
   std::vector<float> sorted(size_t(count) * 12);
-  for (uint32_t i = 0; i < count; ++i) std::memcpy(&sorted[12 * size_t(i)], h + 12 * size_t(idx[i]), 12 * sizeof(float));
+  std::vector<uint32_t> idx(count);
+  for (uint32_t i = 0; i < count; ++i) {
+    idx[i] = cen[i].index;
+    std::memcpy(&sorted[12 * size_t(i)], h + 12 * size_t(idx[i]), 12 * sizeof(float));
+  }
   reach = 0.f;
-  for (size_t k = 0; k < sorted.size(); ++k)
-    if (k % 12 >= 3 && std::isfinite(sorted[k])) reach = std::max(reach, std::fabs(sorted[k]));
+  for (size_t t = 0; t < count; ++t)
+    for (int k = 3; k < 12; ++k)
+      if (std::isfinite(sorted[12 * t + k])) reach = std::max(reach, std::fabs(sorted[12 * t + k]));
   reach *= 1.7320509f;
   const size_t total = size_t(leaves) + groups + blocks;
   std::vector<float4> disc(std::max<size_t>(2 * total + leaves, 1));  // the discs, then a vertex of each leaf
   const uint32_t per[3] = {kMeshLeaf, kMeshLeaf * kMeshFan, kMeshLeaf * kMeshFan * kMeshFan}, runs[3] = {leaves, groups, blocks};
+  std::vector<Extent> ext(total);  // of the leaves, then of what they make up
+  for (uint32_t t = 0; t < count; ++t) ext[t / kMeshLeaf].add(&sorted[12 * size_t(t) + 3]);
+  for (uint32_t l = 0; l < leaves; ++l) ext[leaves + l / kMeshFan].add(ext[l]);
+  for (uint32_t g = 0; g < groups; ++g) ext[leaves + groups + g / kMeshFan].add(ext[leaves + g]);
   size_t at = 0;
   for (int lv = 0; lv < 3; ++lv)
-    for (uint32_t r = 0; r < runs[lv]; ++r, at += 2) hostDisc(sorted.data(), r * per[lv], std::min(count, (r + 1) * per[lv]), &disc[at]);
+    for (uint32_t r = 0; r < runs[lv]; ++r, at += 2)
+      hostDisc(sorted.data(), r * per[lv], std::min(count, (r + 1) * per[lv]), ext[at / 2], &disc[at]);
   for (uint32_t l = 0; l < leaves; ++l, ++at) {
     // of a triangle that can be closest: finite and of some area (none: NaN, no bound)
     disc[at] = make_float4(NAN, NAN, NAN, 0.f);

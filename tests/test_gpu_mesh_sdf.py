@@ -331,3 +331,14 @@ def test_prepared_mesh_of_slivers(count):
     got, want = gpu_mesh_sdf(tris, res, total, h, True), oracle.mesh_sdf(tris, res, total, h)
     # the region test of a sliver 3e-5 wide may return any point across it: its width
     assert np.abs(np.abs(got) - np.abs(want)).max() < 2e-4
+
+
+def test_prepared_mesh_of_many_copies():
+    """40 copies of a sphere in one list (12,800 triangles, 40 with each centroid:
+    the preparation's splits are decided by list index alone), the first copy
+    with its normals flipped: equal distances everywhere, the first copy's sign."""
+    base = mesh.icosphere((0.5, 0.5, 0.5), 0.25, 2)
+    tris = np.tile(base, (40, 1))
+    tris[: len(base), 0:3] *= -1.0
+    res, total, h = (16, 16, 16), 16 ** 3, 1 / 16
+    assert_same_sdf(gpu_mesh_sdf(tris, res, total, h, True), oracle.mesh_sdf(tris[: len(base)], res, total, h))
