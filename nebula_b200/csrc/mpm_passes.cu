@@ -166,16 +166,25 @@ __global__ void __launch_bounds__(kThreads) k_bin_canon_particles(uint32_t n, co
 }
 constexpr uint32_t kCanonParticleBlocks = 1184;  // 8 CTAs on each of 148 SMs; every launch whose cells are small pays only their start
 
-// P2G: a warp takes 32 sorted slots, sums the particles that share a cell
-// (mpm_p2g.cuh) and adds each group's 27 nodes to the dense grid.  What bounds it
-// is the reductions to L2: 27 of 16 bytes and 27 of 4 per group, where one
-// thread per particle issued as many per particle.  300,000 particles in cell
-// order: 31 us (bin to grid update of 128^3: 225 -> 102 us a pass, most of the rest
-// the zeroing of the 75 MB grid).
-__global__ void __launch_bounds__(kThreads) k_p2g_dense(SubstepParams P, StatePtrs st, const uint32_t* __restrict__ sorted, uint32_t n,
+// P2G: a warp takes `slots` (a power of two up to 32) sorted slots, sums the
+// particles that share a cell (mpm_p2g.cuh) and adds each group's 27 nodes to the
+// dense grid.  What bounds it is the reductions to L2: 27 of 16 bytes and 27 of 4
+// per group, where one thread per particle issued as many per particle.  300,000
+// particles in cell order: 31 us (bin to grid update of 128^3: 225 -> 102 us a
+// pass, most of the rest the zeroing of the 75 MB grid).
+//
+// A warp's groups come one after another, up to one per slot: with few warps
+// that chain is the pass, and scattered particles in 32 slots a warp were slower
+// than one thread each (4,000 at random: 15.7 -> 16.7 us with the zeroing of a
+// 64^3 grid).  So up to kP2GSmall particles a warp takes 8 slots: 9.7 us there, 8.3
+// instead of 10.4 in cell order; 10,000: 11.1 for 17.1, 9.4 for 10.9.  At 30,000
+// the warps are enough and the groups count: 11.3 for 10.5 in cell order.
+constexpr uint32_t kP2GSmall = 16384;
+__global__ void __launch_bounds__(kThreads) k_p2g_dense(SubstepParams P, StatePtrs st, const uint32_t* __restrict__ sorted, uint32_t n, uint32_t slots,
                                                         float4* gridMom, float* gridMass) {
   __shared__ __align__(16) WarpRows rows[kThreads / 32];
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+  const uint32_t lane = threadIdx.x & 31u, warp = (blockIdx.x * kThreads + threadIdx.x) >> 5;
+  const uint32_t t = lane < slots ? warp * slots + lane : n;
   WarpRows& W = rows[threadIdx.x >> 5];
   uint32_t key = kNoKey;
   bool exact = false;
@@ -301,7 +310,8 @@ cudaError_t launchBinScanExpiryProbe(const SubstepParams& P, const BinBuffers& b
 cudaError_t launchP2GDense(const SubstepParams& P, StatePtrs st, const uint32_t* sorted, uint32_t n, float4* gridMom, float* gridMass,
                            cudaStream_t s, uint64_t* launches) {
   if (n == 0) return cudaSuccess;
-  k_p2g_dense<<<blocksFor(n), kThreads, 0, s>>>(P, st, sorted, n, gridMom, gridMass);
+  const uint32_t slots = n <= kP2GSmall ? 8u : 32u;
+  k_p2g_dense<<<blocksFor(uint64_t(n) * (32u / slots)), kThreads, 0, s>>>(P, st, sorted, n, slots, gridMom, gridMass);
   ++*launches;
   return cudaGetLastError();
 }
