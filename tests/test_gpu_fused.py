@@ -434,3 +434,41 @@ def test_fused_rounds_and_model_sets_equal_the_dense_pipeline(n, flip):
             eng.cleanup()
         assert rel_l2(out[0]["P"][:, :3], out[1]["P"][:, :3]) < 1e-6, name
         assert rel_l2(out[0]["v"][:, :3], out[1]["v"][:, :3]) < 1e-6, name
+
+
+@pytest.mark.parametrize("flip", [-1.0, 0.95], ids=["apic", "flip"])
+@pytest.mark.parametrize("n", [33, 12000])
+def test_fused_strained_state_equals_the_dense_pipeline_and_the_oracle(n, flip):
+    """F and the stress of the fused kernel's instantiations, from a state whose
+    principal stretches are apart (at F = I their axes are rounding), against the
+    dense pipeline and against the oracle, whose P2G is a gather per node and
+    shares nothing with the warps' sums: one substep, 1e-6 for F (8 ulp), 1e-4
+    for the stress (rounding of F over gaps of 0.01 in the stretches)."""
+    res = 96
+    h = float(np.float32(1.0 / res))
+    side = int(np.ceil(n ** (1.0 / 3.0)))
+    pos = S.jittered_lattice(9, 0, (side, side, side), 0.5 * h, (0.3, 0.3, 0.3), 0.2 * h)[:n]
+    vel = np.stack([2.0 * (pos[:, 1] - 0.3), 0.5 * np.sin(9.0 * pos[:, 0]), -1.0 * (pos[:, 2] - 0.3)], 1)
+    kinds = {"elastic": [S.material(S.MAT_ELASTIC, 1e4, 0.3, 1000.0)],
+             "von_mises": [S.material(S.MAT_VON_MISES, 1e4, 0.3, 1000.0, q_max=100.0)],
+             "sand": [S.material(S.MAT_DRUCKER_PRAGER, 1e5, 0.3, 1600.0, M_friction=0.6, q_cohesion=2e3)],
+             "elastic_sand": [S.material(S.MAT_ELASTIC, 1e4, 0.3, 1000.0), S.material(S.MAT_DRUCKER_PRAGER, 1e5, 0.3, 1600.0, M_friction=0.6, q_cohesion=2e3)]}
+    for name, mats in kinds.items():
+        sp = S.StepParams(dt=5e-5, cell_size=h, domain_size=(1.0, 1.0, 1.0), flip_ratio=flip, materials=mats, forces=[S.gravity()])
+        sp.rho0 = float(mats[0]["rho0"])
+        st = S.make_state(pos, np.float32((0.5 * h) ** 3), vel=vel, mat_ids=np.arange(n) * len(mats) // n)
+        for k, stretch in enumerate((0.99, 0.98, 0.97)):
+            st["F%d" % k][:, k] = stretch + 0.002 * np.sin(7.0 * pos[:, (k + 1) % 3])
+        sc = S.Scene(name, sp, st, 1)
+        out = []
+        for pipeline in ("fused", "dense"):
+            eng = engine_for_scene(sc, pipeline=pipeline)
+            eng.run_substeps(sp.dt, 1)
+            out.append(eng.state())
+            eng.cleanup()
+        out.append(oracle_run(sc, 1, mode="ref32" if name == "elastic" else "mixed"))
+        tau = [np.stack([o[f][:, 3] for f in ("F0", "F1", "F2", "B0", "B1", "B2")], 1) for o in out]
+        for k in (1, 2):
+            eF, es = rel_l2(Fm(out[0]), Fm(out[k])), rel_l2(tau[0], tau[k])
+            print("%s against %s: F %.2e stress %.2e" % (name, ("dense", "oracle")[k - 1], eF, es))
+            assert eF < 1e-6 and es < 1e-4, (name, k)
