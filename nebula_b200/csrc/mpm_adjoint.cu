@@ -62,7 +62,8 @@ __device__ __forceinline__ float bspline2h(float d) {
   return 0.0f;
 }
 
-// Grid accessor for g2pParticle over the dense velocity grid (w = mass).
+// Grid accessor for g2pGather over the dense velocity grid (w = mass; the
+// velocity is zero where the mass is below 1e-10).
 struct VelGrid {
   const float4* vel;
   __device__ __forceinline__ bool node(int x, int y, int z, float& m, float3& v, float3& vo) const {
@@ -72,6 +73,10 @@ struct VelGrid {
     v = make_float3(a.x, a.y, a.z);
     vo = v;
     return true;
+  }
+  __device__ __forceinline__ float3 velocity(int x, int y, int z) const {
+    const float4 a = __ldg(vel + mortonEncode(x, y, z));
+    return make_float3(a.x, a.y, a.z);
   }
 };
 
@@ -173,6 +178,13 @@ __global__ void __launch_bounds__(kT) k_fwd_grid(SubstepParams P, float4* acc, f
   });
 }
 
+// The gather keeps the order of its sums, and scales the weight gradients as the
+// adjoint below does when it forms G again.  The engine's factorized gather is
+// 1 to 3% faster here (56,832 particles, 40 substeps forward and backward: 4.64
+// against 4.68 ms; a node test and a division per term: 5.36), but the gradient
+// of a block in floor contact amplifies rounding 10^5-fold: of 1,024 rollouts of
+// 50,000 particles and 200 substeps each, 162 came out further than 2.5e-2 from the
+// float64 gradient with it, 105 with a test and a division per term, 35 so.
 __global__ void __launch_bounds__(kP) k_fwd_g2p(SubstepParams P, St in, St out, const float2* __restrict__ lame, uint32_t n,
                                                 const float4* __restrict__ vel, AdjScalars* sc) {
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -183,9 +195,15 @@ __global__ void __launch_bounds__(kP) k_fwd_g2p(SubstepParams P, St in, St out, 
   Pp.mu_lame = l.x;
   Pp.lambda_lame = l.y;
   float vpic[3], vpo[3], G[3][3], Bn[3][3];
-  int cell[3];
-  // (the velocity grid is zero where a node is lighter than 1e-10)
-  if (!g2pGatherGrid<false>(Pp, s, vel, nullptr, vpic, vpo, G, Bn, cell[0], cell[1], cell[2])) g2pGather(Pp, s, VelGrid{vel}, vpic, vpo, G, Bn);
+  bool inside = true;
+  const float xp[3] = {s.P.x, s.P.y, s.P.z};
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const int c = __float2int_rd(__fdiv_rn(xp[a] - P.worldMin[a], P.cellSize));
+    inside = inside && c >= 1 && c <= P.gridRes[a] - 2;
+  }
+  if (inside) g2pGather<true>(Pp, s, VelGrid{vel}, vpic, vpo, G, Bn);
+  else g2pGather(Pp, s, VelGrid{vel}, vpic, vpo, G, Bn);
   const uint32_t ev = g2pUpdate<kModelsElastic>(Pp, s, P.dt, vpic, vpo, G, Bn);
   const float lo = 1.5f * P.cellSize;
   uint32_t flags = (ev & 1u) ? 1u : 0u;
@@ -383,13 +401,10 @@ __device__ __forceinline__ void storeRows(float4* rows, uint32_t p, const float 
 // G2P adjoint: adjoints of (x', v', B', F', tau') -> adjoint of x (partial), F,
 // mu, lambda, and the grid-velocity adjoint (scattered).
 // What bounds it is the latency of one particle's chain with few warps to cover
-// it: at 214 registers 9 warps fitted an SM, so the 1,563 warps of 50,000
-// particles took two waves; at 168 (six CTAs of 64) they take one.  With the
-// factorized gather in k_fwd_g2p, forward and backward of 100 substeps: 10.2 ->
-// 7.7 ms (8.8 without the other passes' share).  Particles in cell order with
-// per-cell scatters gave 7.3, but on a block in floor contact, whose gradient
-// amplifies rounding 10^5-fold, its runs strayed above 2.5e-2 from the float64
-// gradient 5 times in 16 instead of once.
+// it: at 214 registers 9 warps fitted an SM, at 168 (six CTAs of 64) 12 do.  With
+// the gather of k_fwd_g2p, 40 substeps forward and backward: 30,000 particles 4.4
+// -> 3.9 ms, 56,832 (the last size of one wave) 6.3 -> 4.7, 60,000 6.1 -> 5.4,
+// 200,000 16.5 -> 12.6, 500,000 37.7 -> 29.2.
 __global__ void __launch_bounds__(kP, 6) k_adj_g2p(SubstepParams P, St st, const float2* __restrict__ lame, uint32_t n, const float4* __restrict__ vel,
                                                 AdjPtrs ob, AdjPtrs ib, float4* gadj, float* mub, float* lamb) {
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;

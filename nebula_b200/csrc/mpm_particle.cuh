@@ -173,10 +173,14 @@ __device__ __forceinline__ bool gridNode(const SubstepParams& P, int ix, int iy,
 // ---------------------------------------------------------------- G2P
 // Gather of mpm_g2p.comp:87-118 through a node accessor: vpic, vpic_old,
 // grad v (G) and the APIC B (both GLSL [col][row]).
-template <class Grid>
+// INSIDE: every node of the stencil lies in [0, gridRes), and grid.velocity is
+// zero where a node is lighter than 1e-10.  The same terms in the same order, but
+// no node is skipped by a branch, so all 27 loads are in flight at once, and the
+// weight gradients are scaled by the reciprocal cell size.
+template <bool INSIDE = false, class Grid>
 __device__ __forceinline__ void g2pGather(const SubstepParams& P, const PState& s, const Grid& grid, float vpic[3], float vpo[3], float G[3][3],
                                           float Bn[3][3]) {
-  const float h = P.cellSize;
+  const float h = P.cellSize, invH = 1.0f / h;
   const float xp[3] = {s.P.x, s.P.y, s.P.z};
   int base[3];
 #pragma unroll
@@ -206,15 +210,23 @@ __device__ __forceinline__ void g2pGather(const SubstepParams& P, const PState& 
 #pragma unroll
       for (int ix = 0; ix < 3; ix++) {
         const int nx = base[0] + ix, ny = base[1] + iy, nz = base[2] + iz;
-        if (nx < 0 || ny < 0 || nz < 0 || nx >= P.gridRes[0] || ny >= P.gridRes[1] || nz >= P.gridRes[2]) continue;
-        float mass;
-        float3 vi, vo;
-        if (!grid.node(nx, ny, nz, mass, vi, vo)) continue;
-        if (mass < 1e-10f) continue;
         const float wx = wa[0][ix], wy = wa[1][iy], wz = wa[2][iz];
         const float w = wx * wy * wz;
-        if (w < 1e-12f) continue;
-        const float dw[3] = {__fdiv_rn(ga[0][ix] * wy * wz, h), __fdiv_rn(wx * ga[1][iy] * wz, h), __fdiv_rn(wx * wy * ga[2][iz], h)};
+        float3 vi, vo;
+        if constexpr (INSIDE) {
+          vi = grid.velocity(nx, ny, nz);
+          if (w < 1e-12f) vi = make_float3(0.f, 0.f, 0.f);
+          vo = vi;
+        } else {
+          float mass;
+          if (nx < 0 || ny < 0 || nz < 0 || nx >= P.gridRes[0] || ny >= P.gridRes[1] || nz >= P.gridRes[2]) continue;
+          if (!grid.node(nx, ny, nz, mass, vi, vo)) continue;
+          if (mass < 1e-10f) continue;
+          if (w < 1e-12f) continue;
+        }
+        float dw[3] = {ga[0][ix] * wy * wz, wx * ga[1][iy] * wz, wx * wy * ga[2][iz]};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) dw[a] = INSIDE ? dw[a] * invH : __fdiv_rn(dw[a], h);
         const float r[3] = {xi[0][ix] - xp[0], xi[1][iy] - xp[1], xi[2][iz] - xp[2]};
         const float v3[3] = {vi.x, vi.y, vi.z};
 #pragma unroll

@@ -72,6 +72,33 @@ def test_forward_matches_engine_uniform_E():
     assert rel(got, want) < 1e-5
 
 
+@pytest.mark.parametrize("res", [32, 24])
+def test_forward_gather_at_the_borders(res):
+    """One substep of particles all over the domain, in its border cells (whose
+    stencils leave the grid) and a little outside: the rollout's two gathers
+    against the dense pipeline's, on a cell size that is a power of two and on
+    one that is not.  P2G and G2P sum a few dozen float terms: 1e-6 (8 ulp) of x
+    and F, 1e-5 of B (differences of velocities)."""
+    h = float(np.float32(1.0 / res))
+    rng = np.random.default_rng(res)
+    n = 3000
+    pos = rng.uniform(-0.05, 1.05, (n, 3)).astype(np.float32)
+    sp = S.StepParams(dt=1e-4, cell_size=h, domain_size=(1.0, 1.0, 1.0), flip_ratio=-1.0,
+                      materials=[S.material(S.MAT_ELASTIC, 1e4, 0.3, 1000.0)], forces=[S.gravity()])
+    sp.rho0 = 1000.0
+    st = S.make_state(pos, np.float32((0.5 * h) ** 3), vel=rng.normal(0.0, 1.0, (n, 3)).astype(np.float32))
+    sc = S.Scene("borders", sp, st, 1, extra={"E": np.full(n, 1e4, np.float32), "target": np.zeros(3), "nu": 0.3, "rho0": 1000.0})
+    roll = Rollout.for_scene(sc)
+    x0, v0, E = inputs(sc)
+    roll.forward(x0, v0, E, sc.extra["target"])
+    torch.cuda.synchronize()
+    eng = engine_for_scene(sc, pipeline="dense")
+    eng.run_substeps(sp.dt, 1)
+    want = eng.state()
+    for f, tol in (("P", 1e-6), ("F0", 1e-6), ("F1", 1e-6), ("F2", 1e-6), ("B0", 1e-5), ("B1", 1e-5), ("B2", 1e-5)):
+        assert rel(roll.final_state(f)[:, :3], want[f][:, :3]) < tol, f
+
+
 FREE = dict(SMALL, y0_cells=12.0)  # the same block in free fall: no contact during the rollout
 
 
