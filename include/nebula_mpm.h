@@ -372,7 +372,10 @@ int nebula_mpm_export_brick_bins(nebula_mpm* e, uint32_t* numBricks, uint32_t* b
  * NULL).  Scenes are added before the first step; the layout is fixed after
  * it.  Substep k of a step uses collider set min(k, trackLen-1) of each
  * scene's collider track, which is how a host moves a collider every
- * substep (the reference re-uploads ColliderSet between dispatches). */
+ * substep (the reference re-uploads ColliderSet between dispatches).
+ * With its own graphs off, a step may be captured into a graph of the caller's
+ * under the conditions of nebula_mpm_step (an even number of substeps, after one
+ * uncaptured step, no setter between replays); with them on CUDA refuses it. */
 typedef struct nebula_mpm_batch nebula_mpm_batch;
 typedef struct nebula_mpm_batch_config {
   uint32_t maxScenes;     /* scene table capacity (<= 65536) */

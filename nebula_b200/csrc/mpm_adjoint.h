@@ -4,7 +4,7 @@
 // Setting: APIC transfer, ELASTIC (Hencky) material with a per-particle
 // Young's modulus, uniform rho0 and nu, gravity, the grid wall band; no
 // colliders or SDF.  The forward substep is the engine's own (same device
-// functions: p2gParticle, gridNode, g2pParticle) on a dense Morton grid in
+// functions: p2gParticle, gridNode, g2pGather, g2pUpdate) on a dense Morton grid in
 // particle order.  Loss: |COM(x_T) - target|^2 with COM mass-weighted.
 // Backward: reverse-mode adjoint of G2P, grid update and P2G, checkpoints
 // every `checkpointEvery` substeps, each segment recomputed with its states

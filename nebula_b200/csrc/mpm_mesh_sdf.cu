@@ -353,10 +353,10 @@ __global__ void __launch_bounds__(kThreads) k_mesh_sdf(const float4* __restrict_
 //      into shared memory four at a time, one triangle per lane, and every lane
 //      walks the 32 triangles, computing closest points for those whose disc
 //      comes nearer than its bound.
-// What bounds it is arithmetic (20,480-triangle sphere at 128^3: 1.51 ms, where
-// clusters of 32 with bounding spheres took 4.09).  Without step 2 a warp
-// inside a closed mesh, where many leaves are almost equally far, walked 518
-// triangles on average.
+// What bounds it is arithmetic (a bumpy sphere of 20,480 triangles moved to a new
+// pose, 128^3: 1.50 ms, where clusters of 32 with bounding spheres took 4.3).
+// Without step 2 a warp inside a closed mesh, where many leaves are almost equally
+// far, walked 518 triangles on average.
 // The discs are not posed: the cell goes to the mesh frame by the inverse
 // pose, and `pad` covers the rounding of that (and a quaternion off unit
 // length).  Triangles are visited out of list order, so a tie in distance
@@ -810,8 +810,8 @@ void selectFront(std::vector<Centroid>& t, size_t lo, size_t mid, size_t hi, int
 // Order of the triangles: median splits of the centroids along their longest
 // extent, cut at multiples of a block, then a group, then a leaf, so that the
 // runs of every level are compact.  (Runs of a Morton order jump between
-// distant patches of a surface and make wide leaves: 2.41 ms on the
-// 20,480-triangle sphere at 128^3, against 1.51.)
+// distant patches of a surface and make wide leaves: 2.41 ms where median splits
+// give 1.50.)
 // t[t0, t1); ties by list index, so the runs depend on the mesh alone.  The
 // halves are independent: those of the first `forks` splits of a large mesh go to
 // threads of their own.

@@ -102,13 +102,7 @@ __device__ __forceinline__ void p2gNodeTermXYZ(const float4 X, const float4 Y, c
 
 // Contribution of a usual-form row to its stencil node (dx, dy, dz).
 __device__ __forceinline__ void p2gNodeTerm(const float4* __restrict__ row, int dx, int dy, int dz, float acc[4]) {
-  const float4 X = row[dx], Y = row[3 + dy], Z = row[6 + dz];
-  const float wyz = Y.w * Z.w;
-  const float wxz = X.w * Z.w, wxy = X.w * Y.w;
-  acc[0] += wyz * X.x + wxz * Y.x + wxy * Z.x;
-  acc[1] += wyz * X.y + wxz * Y.y + wxy * Z.y;
-  acc[2] += wyz * X.z + wxz * Y.z + wxy * Z.z;
-  acc[3] += X.w * wyz;
+  p2gNodeTermXYZ(row[dx], row[3 + dy], row[6 + dz], acc);
 }
 
 // Contribution of an exact-form row (mass m) to its stencil node, skipped

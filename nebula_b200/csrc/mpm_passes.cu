@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(kThreads) k_bin_canon_particles(uint32_t n, co
     sorted[st + r] = i;
   }
 }
-constexpr uint32_t kCanonParticleBlocks = 1184;  // 8 CTAs on each of 148 SMs; every launch whose cells are small pays only their start
+constexpr uint32_t kCanonParticleBlocks = 1184;  // as many as 148 SMs hold (the blocks stride, so any number is right); a launch whose cells are all small pays only their start
 
 // P2G: a warp takes `slots` (a power of two up to 32) sorted slots, sums the
 // particles that share a cell (mpm_p2g.cuh) and adds each group's 27 nodes to the
