@@ -36,7 +36,8 @@ struct WarpRows {
 // (mpm_p2g.comp:47); the smallest of the 27 weights is the product of the
 // three axis minima, so when that product is below 1e-12 (0.15% of the slope
 // scene's particles: near a cell face in all three axes, or very near one),
-// or the mass is not positive, the row is written in the exact form instead,
+// or the mass is not positive (or so small that 1/m may overflow: far below what
+// the grid update counts as mass), the row is written in the exact form instead,
 // (A_c[d], W_c[d]) for every axis with the mass in `mass`, whose terms carry
 // the shader's test (p2gNodeTermExact).  Returns true for the exact form.
 __device__ __forceinline__ bool p2gRow(const SubstepParams& P, const PState& s, float dtStress, int cx, int cy, int cz, float4* row, float& m) {
@@ -73,7 +74,7 @@ __device__ __forceinline__ bool p2gRow(const SubstepParams& P, const PState& s, 
     bsplineStencil(ds[0], ds[1], ds[2], W[c], G[c]);
   }
   const float wmin = (fminf(W[0][0], fminf(W[0][1], W[0][2])) * fminf(W[1][0], fminf(W[1][1], W[1][2]))) * fminf(W[2][0], fminf(W[2][1], W[2][2]));
-  const bool exact = !(m > 0.f && wmin >= 1e-12f);
+  const bool exact = !(m > 1e-30f && wmin >= 1e-12f);
   const float sx = exact ? 1.0f : m, sa = exact ? 1.0f : 1.0f / m;
 #pragma unroll
   for (int c = 0; c < 3; ++c)

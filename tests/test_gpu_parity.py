@@ -154,6 +154,32 @@ def test_p2g_pass_over_sizes_and_orders(n, order):
     assert rel_l2(gm[:nc, :3], om[:nc, :3]) <= 1e-5 and rel_l2(ga, oa) <= 1e-5
 
 
+@pytest.mark.parametrize("volume", [0.0, 1e-42, 1e-38, 1e-33])
+def test_p2g_of_particles_of_hardly_any_mass(volume):
+    """Particles whose mass (1,000 x volume) is zero, below the smallest float
+    with a finite reciprocal, or tiny share cells with ordinary ones: the grid is
+    the oracle's (1e-5, as above), with no infinity or NaN in it, in the single
+    pass and in the engine's fused path."""
+    sc = S.shear_block()
+    rng = np.random.default_rng(5)
+    n = 600
+    st = S.make_state(rng.uniform(0.45, 0.55, (n, 3)).astype(np.float32), np.float32((0.5 / 64) ** 3), vel=rng.normal(0.0, 1.0, (n, 3)).astype(np.float32))
+    st["P"][::3, 3] = volume
+    sc.state = st
+    o, g = OracleBackend(sc.params, n), GpuBackend(sc.params, n)
+    for be in (o, g):
+        be.upload_particles(st)
+        be.bin()
+        be.p2g()
+    (om, oa), (gm, ga) = o.read_grid(), g.read_grid()
+    nc = sc.params.hash_cells
+    assert np.isfinite(gm[:nc]).all() and np.isfinite(ga).all()
+    assert rel_l2(gm[:nc, :3], om[:nc, :3]) <= 1e-5 and rel_l2(ga, oa) <= 1e-5
+    eng = engine_for_scene(sc)
+    eng.run_substeps(sc.params.dt, 3)
+    assert np.isfinite(eng.state()["P"]).all() and eng.stats()["error_flags"] == 0
+
+
 # ----------------------------------------------------------------------------- grid update
 def test_grid_update_colliders_sdf():
     """Random grid through walls, gravity, all four analytic colliders and a dense SDF."""
