@@ -184,8 +184,7 @@ __device__ __forceinline__ void g2pGather(const SubstepParams& P, const PState& 
   const float xp[3] = {s.P.x, s.P.y, s.P.z};
   int base[3];
 #pragma unroll
-  for (int a = 0; a < 3; ++a)  // (a cell farther out than the clamp has no node on the grid either)
-    base[a] = max(min(__float2int_rd(__fdiv_rn(xp[a] - P.worldMin[a], h)), P.gridRes[a] + 1), -2) - 1;
+  for (int a = 0; a < 3; ++a) base[a] = int(floorf(__fdiv_rn(xp[a] - P.worldMin[a], h))) - 1;
   const bool flip = P.flip_ratio > 0.01f;
 #pragma unroll
   for (int i = 0; i < 3; ++i) vpic[i] = vpo[i] = 0.f;
@@ -210,18 +209,19 @@ __device__ __forceinline__ void g2pGather(const SubstepParams& P, const PState& 
 #pragma unroll
       for (int ix = 0; ix < 3; ix++) {
         const int nx = base[0] + ix, ny = base[1] + iy, nz = base[2] + iz;
-        const float wx = wa[0][ix], wy = wa[1][iy], wz = wa[2][iz];
-        const float w = wx * wy * wz;
+        float mass;
         float3 vi, vo;
-        if constexpr (INSIDE) {
-          vi = grid.velocity(nx, ny, nz);
-          if (w < 1e-12f) vi = make_float3(0.f, 0.f, 0.f);
-          vo = vi;
-        } else {
-          float mass;
+        if constexpr (!INSIDE) {
           if (nx < 0 || ny < 0 || nz < 0 || nx >= P.gridRes[0] || ny >= P.gridRes[1] || nz >= P.gridRes[2]) continue;
           if (!grid.node(nx, ny, nz, mass, vi, vo)) continue;
           if (mass < 1e-10f) continue;
+        }
+        const float wx = wa[0][ix], wy = wa[1][iy], wz = wa[2][iz];
+        const float w = wx * wy * wz;
+        if constexpr (INSIDE) {
+          vo = vi = grid.velocity(nx, ny, nz);
+          if (w < 1e-12f) vo = vi = make_float3(0.f, 0.f, 0.f);
+        } else {
           if (w < 1e-12f) continue;
         }
         float dw[3] = {ga[0][ix] * wy * wz, wx * ga[1][iy] * wz, wx * wy * ga[2][iz]};
