@@ -180,8 +180,8 @@ __global__ void __launch_bounds__(kT) k_fwd_grid(SubstepParams P, float4* acc, f
 
 // The gather keeps the order of its sums, and scales the weight gradients as the
 // adjoint below does when it forms G again.  The engine's factorized gather is
-// 1 to 3% faster here (56,832 particles, 40 substeps forward and backward: 4.64
-// against 4.70 ms; a node test and a division per term: 5.36), but the gradient
+// 1 to 3% faster here (56,832 particles, 40 substeps forward and backward: 4.67
+// against 4.71 ms; a node test and a division per term: 5.36), but the gradient
 // of a block in floor contact amplifies rounding 10^5-fold: of 1,024 rollouts of
 // 50,000 particles and 200 substeps each, 162 came out further than 2.5e-2 from the
 // float64 gradient with it, 105 with a test and a division per term, 80 so.
