@@ -740,7 +740,7 @@ __device__ __forceinline__ void g2p2gRound(const SubstepParams& P, WarpRows& W, 
 // CTAs: staged 6^3 velocities, an 8^3 shared accumulation tile, two barriers
 // per brick.  A warp then waited for the slowest of its CTA -- the largest
 // stall -- and a scene of 160 bricks left most warps idle.)  What bounds it is
-// instruction issue and its latencies (59% of cycles issue on 1,000,000
+// instruction issue and its latencies (60% of cycles issue on 1,000,000
 // Drucker-Prager particles; L1 loads are the largest stall).  Per launch, bricks ->
 // rounds, before the changes whose figures stand at gatherOutside and inStep:
 // 8,000 elastic particles 26 -> 19 us, 85,184 Von Mises under FLIP 78 -> 38,
