@@ -497,12 +497,13 @@ uint32_t nebula_mpm_domain_n_groups(uint32_t cells);
 int nebula_mpm_mesh_sdf(const float* dTris, uint32_t nTris, const uint32_t realRes[3], uint32_t totalCells, float cellSize, float* dSdf,
                         void* stream);
 /* A mesh prepared on the device for repeated SDF builds (a moving obstacle):
- * triangles sorted by the Morton code of their centroids and grouped in
- * clusters of 32 with bounding spheres, so that the build culls clusters
- * before triangles.  Same result as nebula_mpm_mesh_sdf on the same list
- * (ties in distance go to the earlier triangle of the list).  tris: n host
+ * triangles ordered by median splits (on several host threads for large meshes)
+ * into a tree of runs with bounding discs, so that the build visits only the
+ * triangles that some cell needs.  Same result as nebula_mpm_mesh_sdf on the same
+ * list (ties in distance go to the earlier triangle of the list).  tris: n host
  * records of 12 floats (normal, v0, v1, v2).  Used by
- * nebula_mpm_set_collider_mesh / _pose. */
+ * nebula_mpm_set_collider_mesh / _pose.  A pose's rotation is a unit quaternion;
+ * one off unit length is applied as it is, and widens the search. */
 typedef struct nebula_mpm_mesh nebula_mpm_mesh;
 int nebula_mpm_mesh_create(const float* tris, uint32_t n, nebula_mpm_mesh** out);
 int nebula_mpm_mesh_destroy(nebula_mpm_mesh* m);

@@ -736,10 +736,11 @@ __device__ __forceinline__ void g2p2gRound(const SubstepParams& P, WarpRows& W, 
 // Warps take rounds of 32 sorted slots, `gridDim x warps` apart, and use nothing
 // of one another's work (the CTAs of large scenes start their rounds together,
 // below): no brick owns a CTA, so a scene of few or unevenly filled bricks spreads
-// over the SMs as evenly as its rounds do, and a CTA has no staging or tile flush.  (The kernel used to hand particle bricks to
-// CTAs: staged 6^3 velocities, an 8^3 shared accumulation tile, two barriers
-// per brick.  A warp then waited for the slowest of its CTA -- the largest
-// stall -- and a scene of 160 bricks left most warps idle.)  What bounds it is
+// over the SMs as evenly as its rounds do, and a CTA has no staging or tile
+// flush.  (The kernel used to hand particle bricks to CTAs: staged 6^3 velocities,
+// an 8^3 shared accumulation tile, two barriers per brick.  A warp then waited for
+// the slowest of its CTA -- the largest stall -- and a scene of 160 bricks left
+// most warps idle.)  What bounds it is
 // instruction issue and its latencies (60% of cycles issue on 1,000,000
 // Drucker-Prager particles; L1 loads are the largest stall).  Per launch, bricks ->
 // rounds, before the changes whose figures stand at gatherOutside and inStep:
@@ -749,9 +750,8 @@ __device__ __forceinline__ void g2p2gRound(const SubstepParams& P, WarpRows& W, 
 // cells are many and its reductions with them, but the bricks are emptier still:
 // a substep of 250,000 Drucker-Prager particles on 256^3 takes 91 us at 8 to a
 // cell (bricks: 189), 120 at 2 (210), 127 at 1 (326), and 458 strewn at random over
-// the domain (4,185).  256 threads, 3 CTAs per SM: 80
-// registers with some spills to L1-cached local memory.  MS: the
-// material-model set compiled in.
+// the domain (4,185).  256 threads, 3 CTAs per SM: 80 registers with some spills
+// to L1-cached local memory.  MS: the material-model set compiled in.
 template <bool FLIP, bool BATCH, int MS>
 __global__ void __launch_bounds__(kThreads, 3) k_g2p2g(const __grid_constant__ SubstepParams P0, SceneTable T, StatePtrs cur, const uint32_t* __restrict__ pidCur, StatePtrs nxt,
                                                        uint32_t* __restrict__ pidNxt, uint32_t n, BrickBuffers B, GridBuffers G, float dtStress,

@@ -458,7 +458,7 @@ void MPMEngine::clearCollider() { hasSdf_ = false; }
 
 // setColliderSDF(buildMeshSDF(tris, gridRes, hashCells, cellSize)) (MeshSDF.h:98-132),
 // the SDF built on the GPU straight into the engine's SDF buffer.  The mesh
-// stays on the device, prepared (clustered), for setColliderMeshPose.
+// stays on the device, prepared (as a tree), for setColliderMeshPose.
 void MPMEngine::setColliderMesh(const float* tris, uint32_t n) {
   checkMeshArgs(tris, n);
   prepareHostAccess(false);  // a queued substep or rebuild may still read the old SDF or mesh

@@ -8,7 +8,7 @@
 namespace nebula {
 
 constexpr uint32_t kErrNonFinite = 1u << 1;   // a particle left G2P with a non-finite position
-constexpr uint32_t kErrTileOverflow = 1u << 2; // informational: a particle scattered outside its block tile
+constexpr uint32_t kErrTileOverflow = 1u << 2; // informational, set by no present kernel (leavers are counted instead)
 constexpr uint32_t kErrBinRange = 1u << 3;     // a binning index fell outside [0, n) (follows an expired scan wait)
 
 enum : int { kPhaseBin = 0, kPhaseP2G = 1, kPhaseGrid = 2, kPhaseG2P = 3, kPhaseFused = 4, kPhaseOther = 5 };
