@@ -138,6 +138,11 @@ __device__ __forceinline__ Disc triDisc(const Tri& t, float eps) {
   return d;
 }
 
+// a b - c d with every operation rounded: zero where the products are equal.  A
+// fused multiply-add leaves the rounding of one product, and a triangle with two
+// equal vertices then falls through its edge tests.
+__device__ __forceinline__ float cross2(float a, float b, float c, float d) { return __fsub_rn(__fmul_rn(a, b), __fmul_rn(c, d)); }
+
 // Closest point of triangle (a, a + ab, a + ac) to p (MeshSDF.h:48-78).
 __device__ __forceinline__ void closestOnTriangle(const Tri& t, float px, float py, float pz, float& qx, float& qy, float& qz) {
   const float apx = px - t.ax, apy = py - t.ay, apz = pz - t.az;
@@ -152,7 +157,7 @@ __device__ __forceinline__ void closestOnTriangle(const Tri& t, float px, float 
     qx = t.ax + t.bx; qy = t.ay + t.by; qz = t.az + t.bz;
     return;
   }
-  const float vc = d1 * d4 - d3 * d2;
+  const float vc = cross2(d1, d4, d3, d2);
   if (vc <= 0.f && d1 >= 0.f && d3 <= 0.f) {
     const float v = d1 / (d1 - d3);
     qx = t.ax + v * t.bx; qy = t.ay + v * t.by; qz = t.az + v * t.bz;
@@ -164,13 +169,13 @@ __device__ __forceinline__ void closestOnTriangle(const Tri& t, float px, float 
     qx = t.ax + t.cx; qy = t.ay + t.cy; qz = t.az + t.cz;
     return;
   }
-  const float vb = d5 * d2 - d1 * d6;
+  const float vb = cross2(d5, d2, d1, d6);
   if (vb <= 0.f && d2 >= 0.f && d6 <= 0.f) {
     const float w = d2 / (d2 - d6);
     qx = t.ax + w * t.cx; qy = t.ay + w * t.cy; qz = t.az + w * t.cz;
     return;
   }
-  const float va = d3 * d6 - d5 * d4;
+  const float va = cross2(d3, d6, d5, d4);
   if (va <= 0.f && (d4 - d3) >= 0.f && (d5 - d6) >= 0.f) {  // edge BC (Ericson 5.1.5; left out by MeshSDF.h:76-78)
     const float w = (d4 - d3) / ((d4 - d3) + (d5 - d6));
     qx = t.ax + t.bx + w * (t.cx - t.bx); qy = t.ay + t.by + w * (t.cy - t.by); qz = t.az + t.bz + w * (t.cz - t.bz);
@@ -198,12 +203,12 @@ __device__ __forceinline__ float discBound(const Disc& d, float px, float py, fl
 
 // Whether a (posed) triangle is sure to be as close as its vertices: nine finite
 // coordinates and some area.  (A NaN or an overflow fails the comparison.  With a
-// NaN the closest point is NaN; with hardly any area the region test may return
-// any point of the plane: of 4,000,000 points around triangles 3,000 times as long
-// as wide it gave 11 a point farther than the nearest vertex, by up to 70 times the
-// distance, at 100,000 times 459; at 1,000 times, where the line is, none.)  A list
-// of slivers alone bounds nothing and is walked whole: 1,000 of them 100,000 times
-// as long as wide on 128^3 0.40 -> 2.15 ms.
+// NaN the closest point is NaN; with hardly any area rounding decides the region
+// test, and the point may lie far off: of 4,000,000 points around triangles 100,000
+// times as long as wide 30 got one farther than the nearest vertex, by up to 9
+// times the distance, at 10,000 times 5, at 1,000 times 1; at 500 times, where the
+// line is, none of 40,000,000.)  A list of slivers alone bounds nothing and is
+// walked whole: 1,000 of them 100,000 times as long as wide on 128^3 0.40 -> 2.15 ms.
 __device__ __forceinline__ bool canBeClosest(const float (&v)[12]) {
   const float ax = v[6] - v[3], ay = v[7] - v[4], az = v[8] - v[5], cx = v[9] - v[3], cy = v[10] - v[4], cz = v[11] - v[5];
   const float gx = ay * cz - az * cy, gy = az * cx - ax * cz, gz = ax * cy - ay * cx;

@@ -342,3 +342,28 @@ def test_prepared_mesh_of_many_copies():
     tris[: len(base), 0:3] *= -1.0
     res, total, h = (16, 16, 16), 16 ** 3, 1 / 16
     assert_same_sdf(gpu_mesh_sdf(tris, res, total, h, True), oracle.mesh_sdf(tris[: len(base)], res, total, h))
+
+
+@pytest.mark.parametrize("posed", [False, True])
+@pytest.mark.parametrize("kind", ["a=b", "a=c", "b=c", "point"])
+@pytest.mark.parametrize("count", [1, 30, 300])
+def test_triangles_with_equal_vertices(count, kind, posed):
+    """A third of the triangles have two equal vertices (or three): they are
+    segments (or points), as close as those are, whatever the two products of a
+    region test round to; list and prepared mesh against the oracle."""
+    rng = np.random.default_rng(count)
+    v = rng.uniform(0.2, 0.8, (count, 1, 3)) + rng.normal(0.0, 0.1, (count, 3, 3))
+    i = np.arange(0, count, 3)
+    pairs = {"a=b": [(1, 0)], "a=c": [(2, 0)], "b=c": [(2, 1)], "point": [(1, 0), (2, 0)]}[kind]
+    for dst, src in pairs:
+        v[i, dst] = v[i, src]
+    nrm = np.cross(v[:, 1] - v[:, 0], v[:, 2] - v[:, 0])
+    nrm /= np.maximum(np.linalg.norm(nrm, axis=1, keepdims=True), 1e-30)
+    tris = np.concatenate([nrm[:, None], v], 1).reshape(count, 12).astype(np.float32)
+    t, q = (np.array([0.05, -0.02, 0.03], np.float32), np.array([0.8, 0.36, 0.0, 0.48], np.float32)) if posed else (None, None)
+    res, total, h = (20, 24, 17), 32 ** 3, 1 / 24
+    want = oracle.mesh_sdf(mesh.transform_triangles(tris, t, q) if posed else tris, res, total, h)
+    for prepared in (False, True):
+        got = gpu_mesh_sdf(tris, res, total, h, prepared, t, q)
+        # two triangles that are equally near may differ in sign by rounding: distances alone
+        assert np.abs(np.abs(got) - np.abs(want)).max() < 1e-5, prepared
