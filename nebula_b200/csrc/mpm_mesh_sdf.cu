@@ -207,8 +207,9 @@ __device__ __forceinline__ float discBound(const Disc& d, float px, float py, fl
 // test, and the point may lie far off: of 4,000,000 points around triangles 100,000
 // times as long as wide 30 got one farther than the nearest vertex, by up to 9
 // times the distance, at 10,000 times 5, at 1,000 times 1; at 500 times, where the
-// line is, none of 40,000,000.)  A list of slivers alone bounds nothing and is
-// walked whole: 1,000 of them 100,000 times as long as wide on 128^3 0.40 -> 2.15 ms.
+// line is, 1 of 40,000,000, by 0.8 of it.)  A list of slivers alone bounds nothing
+// and is walked whole: 1,000 of them 100,000 times as long as wide on 128^3 0.40 ->
+// 2.15 ms.
 __device__ __forceinline__ bool canBeClosest(const float (&v)[12]) {
   const float ax = v[6] - v[3], ay = v[7] - v[4], az = v[8] - v[5], cx = v[9] - v[3], cy = v[10] - v[4], cz = v[11] - v[5];
   const float gx = ay * cz - az * cy, gy = az * cx - ax * cz, gz = ax * cy - ay * cx;
